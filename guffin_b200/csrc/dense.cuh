@@ -168,7 +168,7 @@ struct ChunkProblem {
 struct ChunkProduct {
     ChunkProblem p[3];
     uint32_t problems = 1, rows = 0;
-    uint32_t window = 0, stage_budget = 0;      // filled by the launcher
+    uint32_t window = 0, tiles = 0;             // filled by the launcher; tiles of the problems that are not grouped
     int* error_flag = nullptr;
 };
 int launch_chunk_product(ChunkProduct product, bool f32, cudaStream_t stream);

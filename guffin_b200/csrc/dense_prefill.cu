@@ -100,133 +100,270 @@ __device__ __forceinline__ void chunk_store8(const ChunkProblem& p, uint32_t ind
 // ------------------------------------------------------------------ bf16 products on tcgen05
 
 constexpr uint32_t kWindowMax = 256;                                   // token rows of a tile: the product's N
-constexpr uint32_t kMaxStages = 8;                                     // a stage: 128 weight columns, then the window's token rows, x 64 K
+constexpr uint32_t kPairTile = 2u * kDenseTile;                        // weight columns of a tile: the product's M, half of them a CTA's
+constexpr uint32_t kStages = 6;                                        // a stage: a CTA's 128 weight columns, then its half of the window's rows, x 64 K
+constexpr uint32_t kStageBytes = kDenseTileBytes + kWindowMax / 2u * 128u;
 constexpr uint32_t kEpilogueWarps = 8;
-constexpr uint32_t kStagedLd = kDenseTile + 4u;                        // floats between staged output rows
+constexpr uint32_t kStagedRows = 32;                                   // token rows that go through shared memory at a time on the way out
+constexpr uint32_t kStagedLd = kDenseTile + 4u;                        // floats between them
 constexpr uint32_t kChunkThreads = (kEpilogueWarps + 2u) * 32u;        // the copying and the issuing warp behind them
-constexpr uint32_t kSmemAlone = 208u * 1024u, kSmemPaired = 104u * 1024u;      // stages of a CTA that has its SM alone, or shares it with another
+constexpr uint32_t kChunkSmem = kStages * kStageBytes + kStagedRows * kStagedLd * 4u;
+static_assert(kChunkSmem + 8u * 1024u <= 227u * 1024u, "stages and staged rows do not fit");
 
-// The tensor core's A operand is a tile of 128 weight columns and its B operand a window of up to 256 token rows, so
-// the product's N follows the rows there are (an expert may have few) and accumulator lanes are output columns.
-__global__ void __launch_bounds__(kChunkThreads, 1) chunk_product_kernel(const __grid_constant__ ChunkProduct p) {
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueWarps * 32u) : "memory"); }
+
+// What one CTA of a pair has to do for tile `t`.
+struct ChunkTile {
+    const ChunkProblem* m;
+    uint32_t index, tile, row0, live, n_rows;      // n_rows: the product's N
+    bool mine;                                     // this CTA's half of the columns exists
+    const uint8_t *weight, *rows;
+};
+
+// Tiles are numbered problem by problem, a product's windows of token rows next to one another so that they find its
+// weights in L2.  A grouped problem (experts; the first of its launch) has as many windows as its groups have rows:
+// `windows` holds the number before every group.  Where all indices of a problem read the same rows their 128-column
+// tiles form one list, so that a pair is only half used at its end.
+__device__ __forceinline__ ChunkTile chunk_tile(const ChunkProduct& p, const uint32_t* windows, uint32_t grouped_tiles, uint32_t t, uint32_t rank) {
+    ChunkTile out;
+    uint32_t which = 0, pair, window, rows;
+    if (t < grouped_tiles) {
+        const ChunkProblem& m = p.p[0];
+        const uint32_t pairs = (m.tiles + 1u) / 2u, at = t / pairs;
+        uint32_t low = 0, high = m.count;          // the group with windows[low] <= at < windows[low + 1]
+        while (high - low > 1u) {
+            const uint32_t middle = (low + high) / 2u;
+            if (windows[middle] <= at) low = middle;
+            else high = middle;
+        }
+        const uint32_t mine = windows[low + 1u] - windows[low], local = t - windows[low] * pairs;
+        window = local % mine; pair = local / mine;
+        out.index = low;
+        rows = m.group_rows[low];
+        out.row0 = m.group_start[low] + window * kWindowMax;
+        rows -= window * kWindowMax;
+        out.live = min(kWindowMax, rows);
+    } else {
+        t -= grouped_tiles;
+        while (which + 1u < p.problems && t >= p.p[which + 1u].first_tile) ++which;
+        t -= p.p[which].first_tile;
+        const uint32_t per = (p.rows + p.window - 1u) / p.window;
+        window = t % per; pair = t / per;
+        out.row0 = window * p.window;
+        out.live = min(p.window, p.rows - out.row0);
+        out.index = 0;
+    }
+    const ChunkProblem& m = p.p[which];
+    out.m = &m;
+    if (!m.group_rows) {
+        if (m.a_block_stride == 0u) {              // one list of tiles
+            const uint32_t last = m.tiles * m.count - 1u, line = 2u * pair + rank;
+            out.mine = line <= last;
+            out.index = min(line, last) / m.tiles;
+            out.tile = min(line, last) % m.tiles;
+        } else {
+            const uint32_t pairs = (m.tiles + 1u) / 2u;
+            out.index = pair / pairs;
+            pair %= pairs;
+        }
+    }
+    if (m.group_rows || m.a_block_stride != 0u) {
+        const uint32_t line = 2u * pair + rank;
+        out.mine = line < m.tiles;
+        out.tile = min(line, m.tiles - 1u);
+    }
+    out.n_rows = (out.live + 31u) & ~31u;
+    out.weight = m.weight + out.index * m.weight_stride + (size_t)out.tile * m.k_blocks * kDenseTileBytes;
+    out.rows = static_cast<const uint8_t*>(m.a.data) + (size_t)(m.a_block0 + out.index * m.a_block_stride) * m.a.capacity * 128u + (size_t)out.row0 * 128u;
+    return out;
+}
+
+// Two CTAs (a cluster) share a tile of 256 weight columns (the tensor core's A, a CTA's half each) x a window of up to 256
+// token rows (its B, half of them copied by each CTA), so the product's N follows the rows there are (an expert may have
+// few) and accumulator lanes are output columns.  Per 64 K and SM that is 32 KB of copies for 512 tensor cycles, where one
+// CTA with the whole window copied 48 KB and was held up by what L2 delivers.  One pair per two SMs, tile after tile: the
+// accumulators have two sets of 256 columns, so a tile's output runs under the next tile's products.
+//
+// Bound by the tensor core (512 cycles per 64 K and pair tile) and just above it by L2 (66 bytes per cycle and SM measured
+// in 16 KB copies: 490 cycles).  Measured, TFLOP/s, beside the one-CTA form this replaced: 2048 rows x 3840 x 30720: 1437;
+// 1024 x 2048 x 16384: 1015 (840); 1024 x 8192 x 2048: 706 (590).  Waits on barriers that the other CTA arrives at must not
+// acquire at cluster scope: each such poll costs a cache invalidation (the first case took 2.6 times as long), and the
+// copies and products are ordered by the barriers themselves.
+//
+// Warps 0-7 write outputs, one thread of warp 8 requests copies, one thread of warp 9 issues the products (rank 0) or
+// passes on that its CTA's copies have landed (rank 1).  Every wait is bounded; a CTA that gives up raises both CTAs'
+// abort words, and both always reach the cluster's barriers.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kChunkThreads, 1) chunk_product_kernel(const __grid_constant__ ChunkProduct p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t tmem_slot, abort_flag;
-    __shared__ __align__(8) uint64_t full[kMaxStages];                  // copies landed (bytes)
-    __shared__ __align__(8) uint64_t free_bar[kMaxStages];              // the stage's products have finished
-    __shared__ __align__(8) uint64_t done_bar[1];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const volatile uint32_t* abort = &abort_flag;
+    __shared__ uint32_t windows[kMaxExperts + 1u];
+    __shared__ __align__(8) uint64_t full[kStages];                     // this CTA's copies landed (bytes)
+    __shared__ __align__(8) uint64_t peer_full[kStages];                // rank 0: the other CTA's have
+    __shared__ __align__(8) uint64_t free_bar[kStages];                 // the stage's products have finished
+    __shared__ __align__(8) uint64_t sums_full[2], sums_free[2];        // a set of accumulators is complete; rank 0: read by both CTAs
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, rank = cluster_rank();
+    volatile uint32_t* abort = &abort_flag;
 
-    uint32_t which = 0;
-    while (which + 1u < p.problems && blockIdx.x >= p.p[which + 1u].first_tile) ++which;
-    const ChunkProblem& m = p.p[which];
-    const uint32_t index = (blockIdx.x - m.first_tile) / m.tiles, tile = (blockIdx.x - m.first_tile) % m.tiles;
-    const uint32_t start = m.group_start ? m.group_start[index] : 0u, rows = m.group_rows ? m.group_rows[index] : p.rows;
-    const uint32_t first_row = blockIdx.y * p.window;
-    if (first_row >= rows) return;
-    const uint32_t live = min(p.window, rows - first_row), n_rows = (live + 15u) & ~15u, row0 = start + first_row;
-    const uint8_t* weight = m.weight + index * m.weight_stride + (size_t)tile * m.k_blocks * kDenseTileBytes;
-    const uint8_t* rows_at = static_cast<const uint8_t*>(m.a.data) + (size_t)(m.a_block0 + index * m.a_block_stride) * m.a.capacity * 128u + (size_t)row0 * 128u;
-
-    const uint32_t stage_bytes = kDenseTileBytes + n_rows * 128u, stages = min(kMaxStages, p.stage_budget / stage_bytes);
-    uint32_t tmem_columns = 32u;
-    while (tmem_columns < n_rows) tmem_columns *= 2u;
     if (tid == 0) {
         abort_flag = 0u;
-        for (uint32_t i = 0; i < kMaxStages; ++i) { mbar_init(&full[i], 1); mbar_init(&free_bar[i], 1); }
-        mbar_init(done_bar, 1);
+        for (uint32_t i = 0; i < kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&peer_full[i], 1); mbar_init(&free_bar[i], 1); }
+        for (uint32_t i = 0; i < 2u; ++i) { mbar_init(&sums_full[i], 1); mbar_init(&sums_free[i], 2u * kEpilogueWarps); }
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(&tmem_slot, tmem_columns);
+    const bool grouped = p.p[0].group_rows != nullptr;
+    if (warp == 1u && grouped) {                                        // windows before every group
+        uint32_t before = 0;
+        for (uint32_t first = 0; first < p.p[0].count; first += 32u) {
+            const uint32_t e = first + lane;
+            uint32_t sum = e < p.p[0].count ? (p.p[0].group_rows[e] + kWindowMax - 1u) / kWindowMax : 0u;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const uint32_t other = __shfl_up_sync(0xffffffffu, sum, offset);
+                if (lane >= (uint32_t)offset) sum += other;
+            }
+            if (e < p.p[0].count) windows[e + 1u] = before + sum;
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) windows[0] = 0u;
+    }
+    __syncwarp();
+    if (warp == 0) tmem_alloc_pair(&tmem_slot, 2u * kWindowMax);
     tc_fence_before_sync();
     __syncthreads();
+    cluster_sync();                                                     // the other CTA's barriers are ready too
     tc_fence_after_sync();
-    const uint32_t tmem = tmem_slot, steps = m.k_blocks;
+    const uint32_t tmem = tmem_slot;
+    const uint32_t grouped_tiles = grouped ? windows[p.p[0].count] * ((p.p[0].tiles + 1u) / 2u) : 0u, total = grouped_tiles + p.tiles;
+    const uint32_t first = blockIdx.x / 2u, pairs = gridDim.x / 2u;
     bool ok = true;
+    auto give_up = [&]() {
+        ok = false;
+        abort_flag = 1u;
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_address(&abort_flag, rank ^ 1u)), "r"(1u) : "memory");
+    };
 
+    // The copying and the issuing warp run their loops with all lanes, and one elected lane issues: the copy and product
+    // instructions take their operands from uniform registers, and in a branch of a single thread every one of them costs
+    // about 50 cycles more.
     if (warp == kEpilogueWarps) {
-        if (lane == 0) {
-            uint32_t requested = 0;
-            for (uint32_t step = 0; step < steps; ++step) {
-                const uint32_t stage = step % stages, use = step / stages;
-                if (use > 0u && !wait_or_abort(&free_bar[stage], (use - 1u) & 1u, abort)) { ok = false; break; }
-                uint8_t* at = smem + stage * stage_bytes;
-                mbar_expect_tx(&full[stage], kDenseTileBytes + n_rows * 128u);
-                bulk_load(at, weight + (size_t)step * kDenseTileBytes, kDenseTileBytes, &full[stage]);
-                bulk_load(at + kDenseTileBytes, rows_at + (size_t)step * m.a.capacity * 128u, n_rows * 128u, &full[stage]);
-                requested = step + 1u;
-            }
-            if (!ok || !wait_or_abort(done_bar, 0u, abort)) {
-                // Copies already requested get a bounded chance to land before the shared memory is released.
-                ok = false;
-                abort_flag = 1u;
-                for (uint32_t step = requested > stages ? requested - stages : 0u; step < requested; ++step)
-                    mbar_wait(&full[step % stages], (step / stages) & 1u, 1u << 16);
+        uint32_t stage = 0, parity = 1u, issued = 0;                    // parity: of the phase of free_bar that the next use waits for (the first use passes)
+        for (uint32_t t = first; t < total && ok; t += pairs) {
+            const ChunkTile tile = chunk_tile(p, windows, grouped_tiles, t, rank);
+            // This CTA's half of the window; rows behind the last (in eights) are not copied, nor their sums read.
+            const uint32_t half = tile.n_rows / 2u, from = rank * half, present = (tile.live + 7u) & ~7u;
+            const uint32_t row_bytes = present > from ? min(half, present - from) * 128u : 0u, steps = tile.m->k_blocks;
+            const size_t row_step = (size_t)tile.m->a.capacity * 128u;
+            const uint8_t *weight = tile.weight, *rows = tile.rows + (size_t)from * 128u;
+            for (uint32_t k = 0; k < steps; ++k) {
+                if (!wait_or_abort(&free_bar[stage], parity, abort)) { give_up(); break; }
+                if (elect_one()) {
+                    uint8_t* at = smem + stage * kStageBytes;
+                    mbar_expect_tx(&full[stage], kDenseTileBytes + row_bytes);
+                    bulk_load(at, weight, kDenseTileBytes, &full[stage]);
+                    if (row_bytes) bulk_load(at + kDenseTileBytes, rows, row_bytes, &full[stage]);
+                }
+                __syncwarp();
+                weight += kDenseTileBytes;
+                rows += row_step;
+                ++issued;
+                if (++stage == kStages) { stage = 0; parity ^= 1u; }
             }
         }
+        // Copies requested and not waited for by anybody get a bounded chance to land before the memory is released.
+        for (uint32_t i = issued > kStages ? issued - kStages : 0u; i < issued; ++i) mbar_wait(&full[i % kStages], (i / kStages) & 1u, ok ? kMbarWaitLimit : 1u << 16);
     } else if (warp == kEpilogueWarps + 1u) {
-        if (lane == 0) {
-            const uint32_t instruction = mma_instruction(kDenseTile, n_rows);
-            for (uint32_t step = 0; step < steps; ++step) {
-                const uint32_t stage = step % stages;
-                if (!wait_or_abort(&full[stage], (step / stages) & 1u, abort)) { ok = false; break; }
-                tc_fence_after_sync();
-                const uint32_t at = smem_u32(smem + stage * stage_bytes);
-#pragma unroll
-                for (uint32_t kk = 0; kk < kDenseBlockK / 16u; ++kk)
-                    mma_bf16(tmem, operand_descriptor(at + kk * 256u), operand_descriptor(at + kDenseTileBytes + kk * 256u), instruction, (step | kk) != 0u ? 1u : 0u);
-                mma_commit(&free_bar[stage]);
-            }
-            if (ok) mma_commit(done_bar);
-            else abort_flag = 1u;
-        }
-    } else {
-        if (!wait_or_abort(done_bar, 0u, abort)) { ok = false; if (lane == 0) abort_flag = 1u; }
-    }
-    const bool failed = __syncthreads_or(ok ? 0 : 1) != 0;
-    // Output, 64 token rows at a time: the accumulators go through shared memory (the stages are free again), so that a
-    // thread holds eight neighbouring columns of a row.
-    float* staged = reinterpret_cast<float*>(smem);                     // [64][kStagedLd]
-    for (uint32_t c0 = 0; c0 < live && !failed; c0 += 64u) {
-        if (warp < kEpilogueWarps) {
-            // Warp w reads accumulator lanes 32 (w % 4) .. + 31, i.e. output columns; a warp's accumulator columns are token rows.
-            tc_fence_after_sync();
-            const uint32_t quarter = warp & 3u, c = c0 + (warp >> 2) * 32u;
-            if (c < live) {
-                float v[32];
-                tmem_load_32(tmem + ((quarter * 32u) << 16) + c, v);
-#pragma unroll
-                for (uint32_t i = 0; i < 32u; ++i) staged[((warp >> 2) * 32u + i) * kStagedLd + quarter * 32u + lane] = v[i];
-            }
-            tc_fence_before_sync();
-        }
-        __syncthreads();
-        const bool paired = paired_chunk(m.output);
-        const uint32_t octets = paired ? 8u : 16u, count = min(64u, live - c0) * octets;
-#pragma unroll 1
-        for (uint32_t i = tid; i < count; i += kChunkThreads) {
-            const uint32_t r = i / octets, octet = i % octets, row = row0 + c0 + r;
-            const float* src = staged + r * kStagedLd + octet * (paired ? 16u : 8u);
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j += 4) *reinterpret_cast<float4*>(v + j) = *reinterpret_cast<const float4*>(src + j);
-            if (!paired) {
-                const uint32_t n = tile * kDenseTile + octet * 8u;
-                if (n < m.n) chunk_store8(m, index, row, n, v);
+        uint32_t stage = 0, parity = 0, count = 0;
+        const uint64_t first_a = operand_descriptor(smem_u32(smem)), first_b = operand_descriptor(smem_u32(smem) + kDenseTileBytes);
+        for (uint32_t t = first; t < total && ok; t += pairs, ++count) {
+            const ChunkTile tile = chunk_tile(p, windows, grouped_tiles, t, rank);
+            const uint32_t steps = tile.m->k_blocks;
+            if (rank != 0u) {
+                for (uint32_t k = 0; k < steps; ++k) {
+                    if (!wait_or_abort(&full[stage], parity, abort)) { give_up(); break; }
+                    if (elect_one()) mbar_arrive_at(cluster_address(&peer_full[stage], 0u));
+                    __syncwarp();
+                    if (++stage == kStages) { stage = 0; parity ^= 1u; }
+                }
                 continue;
             }
-            const uint32_t n = tile * (kDenseTile / 2u) + octet * 8u;
-            if (n >= m.n / 2u) continue;
-            const float s = m.row_scale ? m.row_scale[(size_t)row * m.row_scale_ld] : 1.0f;
+            const uint32_t set = count & 1u, instruction = mma_instruction(kPairTile, tile.n_rows), sums = tmem + set * kWindowMax;
+            if (count >= 2u && !wait_or_abort(&sums_free[set], (count / 2u - 1u) & 1u, abort)) { give_up(); break; }
+            tc_fence_after_sync();
+            for (uint32_t k = 0; k < steps; ++k) {
+                if (!wait_or_abort(&full[stage], parity, abort) || !wait_or_abort(&peer_full[stage], parity, abort)) { give_up(); break; }
+                tc_fence_after_sync();
+                if (elect_one()) {
+                    const uint64_t a = first_a + stage * (kStageBytes / 16u), b = first_b + stage * (kStageBytes / 16u);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = chunk_gate(m, v[j] * s, src[8 + j] * s);
-            *reinterpret_cast<uint4*>(static_cast<uint8_t*>(m.result.data) + operand_offset(m.result, row, n)) = bf16_octet(v);
+                    for (uint32_t kk = 0; kk < kDenseBlockK / 16u; ++kk) mma_bf16_pair(sums, a + kk * 16u, b + kk * 16u, instruction, (k | kk) != 0u ? 1u : 0u);
+                    mma_commit_pair(&free_bar[stage]);
+                    if (k + 1u == steps) mma_commit_pair(&sums_full[set]);
+                }
+                __syncwarp();
+                if (++stage == kStages) { stage = 0; parity ^= 1u; }
+            }
         }
-        __syncthreads();
+    } else {
+        // Output, 32 token rows at a time: the accumulators go through shared memory, so that a thread holds eight
+        // neighbouring columns of a row.
+        float* staged = reinterpret_cast<float*>(smem + kStages * kStageBytes);      // [kStagedRows][kStagedLd]
+        const uint32_t quarter = warp & 3u, lanes = (quarter * 32u) << 16, half = (warp >> 2) * 16u;
+        uint32_t count = 0;
+        for (uint32_t t = first; t < total; t += pairs, ++count) {
+            const ChunkTile tile = chunk_tile(p, windows, grouped_tiles, t, rank);
+            const ChunkProblem& m = *tile.m;
+            const uint32_t set = count & 1u, sums = tmem + set * kWindowMax + lanes;
+            if (warp == 0u && !wait_or_abort(&sums_full[set], (count / 2u) & 1u, abort)) give_up();
+            __syncwarp();
+            // All warps go on or none (they share barriers below).
+            uint32_t any;
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                         : "=r"(any) : "r"(ok ? 0u : 1u), "n"(kEpilogueWarps * 32u) : "memory");
+            if (any) { ok = false; break; }
+            tc_fence_after_sync();
+            const bool paired = paired_chunk(m.output);
+            for (uint32_t c0 = 0; c0 < tile.live; c0 += kStagedRows) {
+                float v[16];
+                tmem_load_16(sums + c0 + half, v);
+                if (c0 + kStagedRows >= tile.live) {                    // this warp's last read of the set
+                    tc_fence_before_sync();
+                    if (lane == 0) mbar_arrive_at(cluster_address(&sums_free[set], 0u));
+                }
+                if (!tile.mine) continue;
+#pragma unroll
+                for (uint32_t i = 0; i < 16u; ++i) staged[(half + i) * kStagedLd + quarter * 32u + lane] = v[i];
+                epilogue_sync();
+                const uint32_t octets = paired ? 8u : 16u, work = min(kStagedRows, tile.live - c0) * octets;
+#pragma unroll 1
+                for (uint32_t i = tid; i < work; i += kEpilogueWarps * 32u) {
+                    const uint32_t r = i / octets, octet = i % octets, row = tile.row0 + c0 + r;
+                    const float* src = staged + r * kStagedLd + octet * (paired ? 16u : 8u);
+                    float o[8];
+#pragma unroll
+                    for (int j = 0; j < 8; j += 4) *reinterpret_cast<float4*>(o + j) = *reinterpret_cast<const float4*>(src + j);
+                    if (!paired) {
+                        const uint32_t n = tile.tile * kDenseTile + octet * 8u;
+                        if (n < m.n) chunk_store8(m, tile.index, row, n, o);
+                        continue;
+                    }
+                    const uint32_t n = tile.tile * (kDenseTile / 2u) + octet * 8u;
+                    if (n >= m.n / 2u) continue;
+                    const float s = m.row_scale ? m.row_scale[(size_t)row * m.row_scale_ld] : 1.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) o[j] = chunk_gate(m, o[j] * s, src[8 + j] * s);
+                    *reinterpret_cast<uint4*>(static_cast<uint8_t*>(m.result.data) + operand_offset(m.result, row, n)) = bf16_octet(o);
+                }
+                epilogue_sync();
+            }
+        }
     }
+    const bool failed = __syncthreads_or(ok ? 0 : 1) != 0;
     if (failed && tid == 0) atomicExch(p.error_flag, 1);
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, tmem_columns);
+    __syncwarp();
+    tc_fence_before_sync();
+    cluster_sync();                                                     // nobody reads the other CTA's shared memory or accumulators any more
+    tc_fence_after_sync();
+    if (warp == 0) tmem_dealloc_pair(tmem, 2u * kWindowMax);
 }
 
 // ------------------------------------------------------------------ f32 products
@@ -535,6 +672,7 @@ int launch_chunk_product(ChunkProduct p, bool f32, cudaStream_t stream) {
     for (uint32_t i = 0; i < p.problems; ++i) {
         ChunkProblem& m = p.p[i];
         if (!m.weight || !m.a.data || m.n == 0 || m.k == 0 || m.count == 0 || m.a.f32 != (f32 ? 1u : 0u)) return fail(GF_ERR_INVALID, "chunk product: bad problem");
+        if (m.group_rows && (!m.group_start || (!f32 && (i != 0u || m.count > kMaxExperts)))) return fail(GF_ERR_INVALID, "chunk product: bad groups");
         m.k_blocks = (m.k + kDenseBlockK - 1u) / kDenseBlockK;
         if ((m.a_block0 + (m.count - 1u) * m.a_block_stride + m.k_blocks) * kDenseBlockK > m.a.k_pad) return fail(GF_ERR_INVALID, "chunk product: the operand is narrower than K");
         if (!m.group_rows && p.rows > m.a.capacity) return fail(GF_ERR_INVALID, "chunk product: more rows than the operand holds");
@@ -545,17 +683,35 @@ int launch_chunk_product(ChunkProduct p, bool f32, cudaStream_t stream) {
     if (f32) {
         p.window = 64u;
         chunk_product_f32_kernel<<<dim3(total, (p.rows + 63u) / 64u), 256, 0, stream>>>(p);
-    } else {
-        // The widest window of rows that still gives most SMs a tile.
-        p.window = kWindowMax;
-        while (p.window > 64u && (uint64_t)total * ((p.rows + p.window - 1u) / p.window) * 5u < (uint64_t)sm_count() * 4u) p.window /= 2u;
-        static std::once_flag once[64];
-        const int status = allow_smem(chunk_product_kernel, once, kSmemAlone);
-        if (status != GF_OK) return status;
-        // Many tiles: two CTAs share an SM, so that one's start and output overlap the other's products.
-        p.stage_budget = (uint64_t)total * ((p.rows + p.window - 1u) / p.window) > 3u * (uint64_t)sm_count() ? kSmemPaired : kSmemAlone;
-        chunk_product_kernel<<<dim3(total, (p.rows + p.window - 1u) / p.window), kChunkThreads, p.stage_budget, stream>>>(p);
+        GF_CUDA(cudaGetLastError());
+        return GF_OK;
     }
+    // Pairs of 128-column tiles, and the window of rows with the least time: waves of tiles x what a K block of one costs,
+    // 2 cycles of the tensor core per row or what its copies take at the 70 bytes per cycle and SM that L2 was seen to
+    // deliver, whichever is more, x the largest K (two K blocks more for a tile's start and output).
+    auto pairs_of = [](const ChunkProblem& m) {
+        return m.group_rows ? 0u : m.a_block_stride == 0u ? (m.tiles * m.count + 1u) / 2u : (m.tiles + 1u) / 2u * m.count;
+    };
+    const uint32_t clusters = (uint32_t)sm_count() / 2u;
+    uint32_t pairs = 0;
+    for (uint32_t i = 0; i < p.problems; ++i) pairs += pairs_of(p.p[i]);
+    uint64_t best = ~0ull;
+    for (uint32_t window = kWindowMax; window >= 32u; window -= 32u) {
+        const uint64_t per = (p.rows + window - 1u) / window, waves = (pairs * per + clusters - 1u) / clusters;
+        const uint64_t block = std::max<uint64_t>(2u * window, (kDenseTileBytes + 64u * window) / 70u);
+        if (waves * block < best) { best = waves * block; p.window = window; }
+    }
+    const uint32_t per = (p.rows + p.window - 1u) / p.window;
+    p.tiles = 0;
+    for (uint32_t i = 0; i < p.problems; ++i) {
+        p.p[i].first_tile = p.tiles;
+        p.tiles += pairs_of(p.p[i]) * per;
+    }
+    static std::once_flag once[64];
+    const int status = allow_smem(chunk_product_kernel, once, kChunkSmem);
+    if (status != GF_OK) return status;
+    const uint32_t grid = p.p[0].group_rows ? clusters : std::min(clusters, p.tiles);
+    chunk_product_kernel<<<2u * grid, kChunkThreads, kChunkSmem, stream>>>(p);
     GF_CUDA(cudaGetLastError());
     return GF_OK;
 }

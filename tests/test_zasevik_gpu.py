@@ -68,6 +68,27 @@ def test_chunk_products(gf, gm, k, n, rows):
         assert rel_l2(y.download(np.float32).reshape(rows, n), operand.astype(np.float64) @ w.T) < bound
 
 
+@pytest.mark.parametrize("k,n,rows", [
+    (64, 8, 1),             # half a pair of tiles, fewer rows than the narrowest product
+    (65, 136, 32),          # two tiles, one K element behind a block
+    (448, 257, 33),         # an odd tile behind a whole pair; more K blocks than stages
+    (128, 384, 256), (384, 640, 257),
+    (4160, 520, 289),
+    (128, 5000, 2049),      # three and more tiles a pair: both sets of accumulators used again
+])
+def test_chunk_product_tiles(gf, gm, k, n, rows):
+    """Borders of tiles, windows and stages.  The tensor core's sums do not round to nearest: 2e-6 at K = 1000, growing with K."""
+    rng = np.random.default_rng(rows)
+    weight, w = packed(gf, gm, rng, k, n)
+    x = rng.standard_normal((rows, k)).astype(np.float32)
+    xd, y = gf.DeviceBuffer.from_numpy(x), gf.DeviceBuffer(rows * n * 4)
+    ws = gf.DeviceBuffer(gf.load().gf_dense_chunk_workspace_bytes(rows, k, SERVING))
+    ws.zero()
+    gf.check(gf.load().gf_dense_chunk_matmul(weight.ptr, xd.ptr, y.ptr, rows, k, n, SERVING, ws.ptr, None))
+    want = gm.bf16_values(gm.bf16_bits(x)).astype(np.float64) @ w.T
+    assert rel_l2(y.download(np.float32).reshape(rows, n), want) < 2e-6 * max(1.0, k / 1000.0)
+
+
 def run_attention(gf, q, cache, first, rows, sink, parts, precision, ring_rows):
     """q [rows, heads, rank] scaled, cache [first + rows, rank]: device result [rows, heads, rank]."""
     heads, rank = q.shape[1:]
