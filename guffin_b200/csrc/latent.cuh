@@ -42,15 +42,20 @@ int launch_latent_merge(const LatentAttention& p, cudaStream_t stream);
 // the latent's rank.  For grouped-query attention: over the cache rows themselves.
 constexpr uint32_t kHeadAttentionMaxDim = 256;
 struct HeadAttention {
-    const __half* q = nullptr;           // [rows][heads][dim_pad], scaled
+    const __half* q = nullptr;           // [rows][heads][dim_pad], scaled; or
+    const float* q32 = nullptr;          // the same in 32 bits, multiplied by q_scale here
+    float q_scale = 1.0f;
     const __half* k = nullptr;           // [positions][kv_heads][dim_pad], positions from 0; with rings: the chunk's own rows
     const __half* v = nullptr;           // [positions][kv_heads][vdim_pad]
-    const StreamRings* rings = nullptr;  // the rows before the chunk, or null
+    const StreamRings* rings = nullptr;  // the rows before the chunk, or
+    const __half *ring_k = nullptr, *ring_v = nullptr;      // the same by address, or neither
     uint32_t ring_mask = 0;
     const uint32_t* position = nullptr;  // of row 0
     const float* sink = nullptr;         // per head, or null
     const float* gate = nullptr;         // [rows][heads], ahead of the sigmoid, or null
     float softcap = 0.0f;                // of the scores; 0: none
+    uint32_t window = 0;                 // a row sees its last `window` positions; 0: all before it
+    int* error_flag = nullptr;           // set when a bounded wait gives up
     uint32_t rows = 0, heads = 0, kv_heads = 0, dim_pad = 0, vdim = 0, vdim_pad = 0;      // pads: multiples of 16
     Operand result;                      // (row, head * vdim + d), bf16 or f32
 };

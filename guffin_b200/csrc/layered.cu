@@ -705,6 +705,7 @@ int Model::chunk_layers(const uint32_t* tokens_host, uint32_t rows, bool logits)
             expansion.rows = positions;
             GF_TRY(run(expansion));
             HeadAttention attention;
+            attention.error_flag = error_flag_;
             attention.q = a.head_q; attention.k = a.keys; attention.v = a.values; attention.position = state_dev_; attention.sink = w.sink;
             attention.rows = rows; attention.heads = attention.kv_heads = m.heads; attention.dim_pad = head_pad; attention.vdim = m.vdim; attention.vdim_pad = value_pad;
             attention.result = heads_out;
@@ -766,6 +767,7 @@ int Model::chunk_layers(const uint32_t* tokens_host, uint32_t rows, bool logits)
         ++launches_;
         if (!f32 && row_head <= kHeadAttentionMaxDim) {
             HeadAttention attention;
+            attention.error_flag = error_flag_;
             attention.q = static_cast<const __half*>(a.prepared_q);
             attention.k = static_cast<const __half*>(a.private_rows[l]); attention.v = static_cast<const __half*>(a.private_values[l]);
             attention.rings = p.rings_dev + l; attention.ring_mask = caches_[l].ring_rows - 1u; attention.position = state_dev_;

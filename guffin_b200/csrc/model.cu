@@ -1069,7 +1069,7 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
         ap.ring_mask = cache.ring_rows - 1u; ap.window = cache.window; ap.scale = c.attention_scale;
         ap.softcap = c.attn_softcap; ap.kv_f16 = c.kv_f16;
         ap.defer_merge = 0u;
-        if (prefill_attention_supported(ap)) GF_TRY(launch_prefill_attention(ap, stream_));
+        if (prefill_attention_supported(ap)) GF_TRY(launch_prefill_attention(ap, nullptr, error_flag_, stream_));
         else GF_TRY(launch_attention(ap, stream_, false));
         GF_TRY(launch_prefill_pack(a.attention_out, a.a_q, rows, qw, stream_));
         uint32_t o_splits = prefill_gemm_splits(w.o.n, w.o.k, w.o.dtype);

@@ -73,10 +73,13 @@ int launch_prefill_norm(const float* x, uint32_t splits, const float* residual, 
 int launch_prefill_geglu(const float* gate, const float* up, uint32_t splits, void* a_out, uint32_t rows, uint32_t k, cudaStream_t stream);
 // x[i][0][row][:] = sum over splits of x[i][split][row][:], for `count` <= 3 matrices of n[i] columns
 int launch_prefill_reduce(float* const* x, const uint64_t* n, uint32_t count, uint32_t splits, uint32_t rows, cudaStream_t stream);
-// Attention of a chunk's rows over ring + private rows of a binary16 cache with 256-wide heads (f32 output
-// [rows][heads * 256]); other shapes go through the row kernels (launch_attention).
-bool prefill_attention_supported(const struct AttentionParams& p);
-int launch_prefill_attention(const struct AttentionParams& p, cudaStream_t stream);
+// Attention of a chunk's rows over ring + private rows of a binary16 cache with 256-wide heads: into `result`, or
+// without one f32 rows [rows][heads * 256] at params.out; other shapes go through the row kernels (launch_attention).
+// error_flag (may be null): set when a bounded wait gives up.
+struct AttentionParams;
+struct Operand;
+bool prefill_attention_supported(const AttentionParams& p);
+int launch_prefill_attention(const AttentionParams& p, const Operand* result, int* error_flag, cudaStream_t stream);
 // a = x (f32 rows of width k)
 int launch_prefill_pack(const float* x, void* a_out, uint32_t rows, uint32_t k, cudaStream_t stream);
 

@@ -22,9 +22,18 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ uint64_t operand_descriptor(uint32_t smem_address) {
     return (uint64_t)((smem_address >> 4) & 0x3fffu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46);
 }
+// The same with other distances, in bytes.  K-major: `along` between the two core matrices (8 rows x 8 K) of a K step,
+// `across` between groups of eight rows.  A B operand whose rows are contiguous (MN-major; a core matrix is 8 K x 8 rows,
+// 16 bytes of eight rows per K): `along` between groups of eight K, `across` between groups of eight rows.
+__device__ __forceinline__ uint64_t operand_descriptor(uint32_t smem_address, uint32_t along, uint32_t across) {
+    return (uint64_t)((smem_address >> 4) & 0x3fffu) | ((uint64_t)(along >> 4) << 16) | ((uint64_t)(across >> 4) << 32) | (1ull << 46);
+}
+constexpr uint32_t kMmaF16 = (1u << 4), kMmaRowsOfB = 1u << 16;      // f32 accumulator, f16 x f16, both K-major; B MN-major instead
+__host__ __device__ constexpr uint32_t mma_instruction_f16(uint32_t m, uint32_t n, uint32_t more = 0) { return kMmaF16 | more | ((n >> 3) << 17) | ((m >> 4) << 24); }
 // Instruction descriptor: f32 accumulator, bf16 x bf16, both operands K-major.
 __host__ __device__ constexpr uint32_t mma_instruction(uint32_t m, uint32_t n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 
+// Operands of the 16-bit type the instruction descriptor names.
 __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -103,6 +112,16 @@ __device__ __forceinline__ void tmem_load_16(uint32_t address, float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_store_16(uint32_t address, const float (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(address), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+          "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+          "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+          "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // Bounded wait that also gives up as soon as another warp of the CTA has.

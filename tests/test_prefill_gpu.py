@@ -122,3 +122,15 @@ def test_prefill_attention_matches_oracle(gf, oracle, base, rows, window, ring_r
         want = oracle.attention_row(q[r], keys[first:p + 1].astype(np.float32), values[first:p + 1].astype(np.float32),
                                     heads, kv_heads, hd, 0.0625, softcap)
         assert np.abs(got[r] - want).max() <= 2e-3 * max(1.0, np.abs(want).max()), (base, r, window)
+
+
+@pytest.mark.parametrize("base,rows,window,ring_rows,heads,kv_heads,softcap", [
+    (0, 1, 0, 8, 2, 1, 0.0),                # one row at the first position: one tile of one key
+    (63, 65, 0, 64, 4, 4, 0.0),             # tile and block borders, one head per KV head
+    (190, 256, 100, 256, 6, 2, 0.0),        # three heads per KV head (not packed), windows that begin inside tiles
+    (30, 129, 64, 64, 8, 1, 30.0),          # eight heads per KV head, a window of a whole tile
+    (500, 40, 1, 512, 2, 2, 0.0),           # every row sees itself alone
+])
+def test_prefill_attention_borders(gf, oracle, base, rows, window, ring_rows, heads, kv_heads, softcap):
+    """Borders of the 128-query blocks and 64-key tiles, for every way heads share a block."""
+    test_prefill_attention_matches_oracle(gf, oracle, base, rows, window, ring_rows, heads, kv_heads, softcap)
