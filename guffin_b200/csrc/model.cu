@@ -1,6 +1,8 @@
 // Resident model plan and block schedule (see model.cuh).
 #include "model.cuh"
 #include "gemv.cuh"
+#include "latent.cuh"
+#include "prompt.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -930,10 +932,16 @@ int Model::prefill(const uint32_t* tokens_host, uint32_t count) {
             return fail(GF_ERR_INVALID, "prompt exceeds the bound context (%u + %u > %u)", position_, count, config_.context);
         for (uint32_t i = 0; i < count; ++i)
             if (tokens_host[i] >= token_vocab()) return fail(GF_ERR_INVALID, "token id %u outside the vocabulary", tokens_host[i]);
-        GF_TRY(ensure_prefill_arena());
         while (done < count - 1u) {
-            const uint32_t rows = std::min(prefill_.chunk_rows, count - 1u - done);
-            GF_TRY(prefill_chunk(tokens_host + done, rows));
+            uint32_t rows = wide_rows(count - 1u - done);
+            if (rows) {
+                GF_TRY(ensure_wide_arena());
+                GF_TRY(prefill_wide(tokens_host + done, rows));
+            } else {
+                GF_TRY(ensure_prefill_arena());
+                rows = std::min(prefill_.chunk_rows, count - 1u - done);
+                GF_TRY(prefill_chunk(tokens_host + done, rows));
+            }
             done += rows;
         }
         GF_TRY(forward(tokens_host + done, 1, kForwardLogits));
@@ -1093,6 +1101,177 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
     }
     GF_TRY(launch_kv_publish(a.publish_layers, c.layers, state_dev_, rows, stream_));
     launches_ += 2;
+    position_ += rows;
+    return GF_OK;
+}
+
+// Decoding all weights to HBM costs a chunk the same whatever its rows, so it pays from a number of rows on (kWideFrom);
+// prompts are cut into equal chunks.  Shards keep the 256-row chunks (their exchange is laid out for those), as do plans
+// whose heads prefill_attention_supported refuses; an f32 cache limits the rows to what the row kernels' workspace allows.
+constexpr uint32_t kWideFrom = 257;
+uint32_t Model::wide_rows(uint32_t left) const {
+    const gf_model_config& c = config_;
+    if (left < kWideFrom || sharded() || c.head_dim != 256u || !caches_[0].rope_rotation) return 0;
+    const uint32_t group = c.heads / c.kv_heads;
+    if (group != 1u && group != 2u && group != 4u) return 0;
+    for (const LayerWeights& w : layers_)
+        for (const PackedMatrix* m : {&w.q, &w.k, &w.v, &w.o, &w.gate, &w.up, &w.down})
+            if (m->n % kPrefillTile || m->k % 128u) return 0;
+    uint32_t most = std::min(kWideRows, (c.context + 15u) & ~15u);
+    if (!c.kv_f16) most = std::min(most, 4096u / c.heads);
+    if (most < kWideFrom) return 0;
+    const uint32_t chunks = (left + most - 1u) / most;
+    return (left + chunks - 1u) / chunks;
+}
+
+int Model::ensure_wide_arena() {
+    WideArena& a = wide_;
+    if (a.rows) return GF_OK;
+    const gf_model_config& c = config_;
+    const uint32_t qw = c.heads * c.head_dim, kvw = c.kv_heads * c.head_dim;
+    uint32_t rows = std::min(kWideRows, (c.context + 15u) & ~15u);
+    if (!c.kv_f16) rows = std::min(rows, 4096u / c.heads);
+    rows = (rows + 15u) & ~15u;
+    uint8_t* bytes = nullptr;
+    auto operand = [&](Operand& o, uint32_t k) -> int {
+        o.capacity = rows; o.k_pad = (k + kDenseBlockK - 1u) / kDenseBlockK * kDenseBlockK; o.f32 = 0u;
+        GF_TRY(device_alloc(allocations_, &bytes, o.bytes()));
+        o.data = bytes;
+        return GF_OK;
+    };
+    GF_TRY(operand(a.hidden, c.hidden));
+    GF_TRY(operand(a.heads, qw));
+    GF_TRY(operand(a.ffn, c.ffn));
+    GF_TRY(device_alloc(allocations_, &a.residual, (size_t)rows * c.hidden));
+    GF_TRY(device_alloc(allocations_, &a.projected, (size_t)rows * c.hidden));
+    GF_TRY(device_alloc(allocations_, &a.raw_q, (size_t)rows * qw));
+    GF_TRY(device_alloc(allocations_, &a.raw_k, (size_t)rows * kvw));
+    GF_TRY(device_alloc(allocations_, &a.raw_v, (size_t)rows * kvw));
+    if (c.kv_f16) GF_TRY(device_alloc(allocations_, &a.query, (size_t)rows * qw));
+    else {
+        GF_TRY(device_alloc(allocations_, &a.query32, (size_t)rows * qw));
+        GF_TRY(device_alloc(allocations_, &a.attention_out, (size_t)rows * qw));
+        GF_TRY(device_alloc(allocations_, &bytes, attention_workspace_bytes(rows, c.heads)));
+        a.attention_ws = bytes;
+        GF_CUDA(cudaMemsetAsync(attention_counters(a.attention_ws, rows, c.heads), 0, (size_t)rows * c.heads * sizeof(uint32_t), stream_));
+    }
+    const size_t row = cache_row_bytes(0);
+    GF_TRY(device_alloc(allocations_, &bytes, row * rows)); a.own_k = bytes;
+    GF_TRY(device_alloc(allocations_, &bytes, row * rows)); a.own_v = bytes;
+    size_t tiles = 0;
+    for (const LayerWeights& w : layers_) {
+        auto total = [](std::initializer_list<const PackedMatrix*> set) { size_t n = 0; for (const PackedMatrix* m : set) n += (size_t)m->n * m->k * 2u; return n; };
+        tiles = std::max({tiles, total({&w.q, &w.k, &w.v}), total({&w.o}), total({&w.gate, &w.up}), total({&w.down})});
+    }
+    GF_TRY(device_alloc(allocations_, &a.tiles, tiles));
+    GF_TRY(device_alloc(allocations_, &a.tokens, rows));
+    a.rows = rows;
+    return GF_OK;
+}
+
+// One wide chunk.  A layer is: norm; decode and multiply Q, K, V; rotation and cache rows; attention; decode and multiply O;
+// norm; decode gate and up side by side and multiply with the gate in the output; decode and multiply down.  Norms and
+// products are those of a layered plan's chunks.
+int Model::prefill_wide(const uint32_t* tokens_host, uint32_t rows) {
+    const gf_model_config& c = config_;
+    WideArena& a = wide_;
+    const uint32_t qw = c.heads * c.head_dim, kvw = c.kv_heads * c.head_dim;
+    const size_t element = c.kv_f16 ? 2u : 4u, row_bytes = kvw * element;
+    GF_CUDA(cudaMemcpyAsync(a.tokens, tokens_host, rows * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));      // pageable: staged by the driver
+    GF_TRY(launch_embedding(token_embd_.dtype, token_embd_.data, c.hidden, token_vocab(), a.tokens, rows, sqrtf((float)c.hidden), a.residual, status_dev_, stream_, false));
+    ++launches_;
+    ChunkNorm norm;
+    norm.residual = a.residual; norm.width = c.hidden; norm.rows = rows; norm.eps = c.rms_eps; norm.result = a.hidden;
+    auto normalise = [&](const float* y, const float* gain0, const float* gain1) -> int {
+        norm.y = y; norm.gain0 = gain0; norm.gain1 = gain1;
+        ++launches_;
+        return launch_chunk_norm(norm, stream_);
+    };
+    // Matrices behind one another in the tile buffer, or two of equal shape with their groups of eight columns in turn.
+    auto multiply = [&](std::initializer_list<const PackedMatrix*> set, bool paired, const Operand& in, std::initializer_list<float*> outs, const Operand* result) -> int {
+        WideDecode decode;
+        ChunkProduct product;
+        product.problems = 0; product.rows = rows; product.error_flag = error_flag_;
+        uint8_t* tiles = a.tiles;
+        auto out = outs.begin();
+        for (const PackedMatrix* m : set) {
+            WideMatrix& d = decode.m[decode.matrices];
+            d.packed = m->data; d.dtype = (uint32_t)m->dtype; d.pairs = (uint32_t)(m->n / 16u); d.units = (uint32_t)(m->k / unit_elements(m->dtype));
+            d.k_blocks = (uint32_t)(m->k / kDenseBlockK); d.tiles = tiles; d.first_warp = decode.warps;
+            d.group_step = paired ? 2u : 1u; d.group_first = paired ? decode.matrices : 0u;
+            decode.warps += d.pairs * d.units;
+            ++decode.matrices;
+            if (paired && decode.matrices == 2u) break;
+            ChunkProblem& p = product.p[product.problems++];
+            p.weight = tiles; p.k = (uint32_t)m->k; p.n = (uint32_t)m->n * (paired ? 2u : 1u); p.a = in;
+            if (paired) { p.output = kChunkGeluGate; p.result = *result; }
+            else { p.out = *out++; p.out_ld = (uint32_t)m->n; tiles += (size_t)m->n * m->k * 2u; }
+        }
+        launches_ += 2;
+        GF_TRY(launch_wide_decode(decode, stream_));
+        return launch_chunk_product(product, false, stream_);
+    };
+    for (uint32_t l = 0; l < c.layers; ++l) {
+        const LayerWeights& w = layers_[l];
+        const LayerCache& cache = caches_[l];
+        const bool last = l + 1u == c.layers;              // nothing behind its cache rows is needed
+        GF_TRY(normalise(l ? a.projected : nullptr, l ? layers_[l - 1].post_ffw_norm : nullptr, w.attn_norm));
+        if (last) GF_TRY(multiply({&w.k, &w.v}, false, a.hidden, {a.raw_k, a.raw_v}, nullptr));
+        else GF_TRY(multiply({&w.q, &w.k, &w.v}, false, a.hidden, {a.raw_q, a.raw_k, a.raw_v}, nullptr));
+        // The chunk's cache rows go straight to their ring slots where these lie behind one another and hold nothing that a
+        // row of the chunk still sees; otherwise to a buffer that is published behind the attention.
+        const uint32_t slot = position_ & (cache.ring_rows - 1u);
+        const bool direct = slot + rows <= cache.ring_rows && (position_ == 0u || cache.window == 0u || rows + cache.window <= cache.ring_rows);
+        void* keys = direct ? static_cast<uint8_t*>(cache.ring_k) + slot * row_bytes : a.own_k;
+        void* values = direct ? static_cast<uint8_t*>(cache.ring_v) + slot * row_bytes : a.own_v;
+        WideRope rope;
+        rope.raw_q = last ? nullptr : a.raw_q; rope.raw_k = a.raw_k; rope.raw_v = a.raw_v;
+        rope.q_norm = c.uses_qk_norm ? w.q_norm : nullptr; rope.k_norm = c.uses_qk_norm ? w.k_norm : nullptr;
+        rope.q = a.query; rope.q32 = a.query32; rope.keys = keys; rope.values = values;
+        rope.position = state_dev_; rope.rotation = cache.rope_rotation; rope.status = status_dev_;
+        rope.rows = rows; rope.heads = c.heads; rope.kv_heads = c.kv_heads; rope.table_rows = c.context + GF_MAX_ROWS;
+        rope.eps = c.rms_eps; rope.scale = c.attention_scale; rope.kv_f16 = c.kv_f16;
+        ++launches_;
+        GF_TRY(launch_wide_rope(rope, stream_));
+        if (!last) {
+            ++launches_;
+            if (c.kv_f16) {
+                HeadAttention attention;
+                attention.q = a.query;
+                attention.k = static_cast<const __half*>(keys); attention.v = static_cast<const __half*>(values);
+                attention.ring_k = static_cast<const __half*>(cache.ring_k); attention.ring_v = static_cast<const __half*>(cache.ring_v);
+                attention.ring_mask = cache.ring_rows - 1u; attention.position = state_dev_; attention.softcap = c.attn_softcap; attention.window = cache.window;
+                attention.error_flag = error_flag_;
+                attention.rows = rows; attention.heads = c.heads; attention.kv_heads = c.kv_heads; attention.dim_pad = attention.vdim = attention.vdim_pad = 256u;
+                attention.result = a.heads;
+                GF_TRY(launch_head_attention(attention, stream_));
+            } else {
+                AttentionParams ap;
+                ap.q = a.query32; ap.ring_k = cache.ring_k; ap.ring_v = cache.ring_v; ap.private_k = keys; ap.private_v = values; ap.out = a.attention_out;
+                ap.partial_out = static_cast<float*>(a.attention_ws);
+                ap.partial_ml = ap.partial_out + (size_t)a.rows * c.heads * kMaxAttentionPartitions * 256u;
+                ap.counters = attention_counters(a.attention_ws, a.rows, c.heads);
+                ap.base_position = state_dev_; ap.rows = rows; ap.heads = c.heads; ap.kv_heads = c.kv_heads; ap.head_dim = c.head_dim;
+                ap.ring_mask = cache.ring_rows - 1u; ap.window = cache.window; ap.scale = c.attention_scale; ap.softcap = c.attn_softcap; ap.kv_f16 = 0;
+                ap.defer_merge = 0u;
+                GF_TRY(launch_attention(ap, stream_, false));
+                ++launches_;
+                GF_TRY(launch_chunk_operand(a.attention_out, rows, qw, a.heads, stream_));
+            }
+        }
+        if (!direct) {
+            ++launches_;
+            GF_TRY(launch_wide_publish(a.own_k, a.own_v, cache.ring_k, cache.ring_v, state_dev_, rows > cache.ring_rows ? rows - cache.ring_rows : 0u, rows,
+                                       cache.ring_rows - 1u, (uint32_t)row_bytes, stream_));
+        }
+        if (last) break;
+        GF_TRY(multiply({&w.o}, false, a.heads, {a.projected}, nullptr));
+        GF_TRY(normalise(a.projected, w.post_attention_norm, w.ffn_norm));
+        GF_TRY(multiply({&w.gate, &w.up}, true, a.hidden, {}, &a.ffn));
+        GF_TRY(multiply({&w.down}, false, a.ffn, {a.projected}, nullptr));
+    }
+    ++launches_;
+    GF_TRY(launch_advance_position(state_dev_, rows, stream_));
     position_ += rows;
     return GF_OK;
 }

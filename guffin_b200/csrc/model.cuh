@@ -256,7 +256,23 @@ private:
     int ensure_prefill_arena();
     int prefill_chunk(const uint32_t* tokens_host, uint32_t rows);
 
-    // Buffers of the 128-row prompt path, allocated when a long prompt first arrives.
+    // Wide prompt chunks (prompt.cuh): how many of the `left` rows of a prompt the next one takes, 0 for none.
+    uint32_t wide_rows(uint32_t left) const;
+    int ensure_wide_arena();
+    int prefill_wide(const uint32_t* tokens_host, uint32_t rows);
+    struct WideArena {
+        uint32_t rows = 0;                                   // at most, per chunk; 0: not allocated
+        Operand hidden, heads, ffn;                          // bf16 operands
+        float *residual = nullptr, *projected = nullptr, *raw_q = nullptr, *raw_k = nullptr, *raw_v = nullptr, *query32 = nullptr;
+        __half* query = nullptr;
+        void *own_k = nullptr, *own_v = nullptr;             // one layer's cache rows of a chunk
+        uint8_t* tiles = nullptr;                            // the decoded weights of one launch
+        void* attention_ws = nullptr;                        // f32 caches
+        float* attention_out = nullptr;
+        uint32_t* tokens = nullptr;
+    } wide_;
+
+    // Buffers of the 256-row prompt path, allocated when a long prompt first arrives.
     struct PrefillArena {
         bool ready = false;
         uint32_t chunk_rows = 0;

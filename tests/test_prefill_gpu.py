@@ -127,10 +127,45 @@ def test_prefill_attention_matches_oracle(gf, oracle, base, rows, window, ring_r
 @pytest.mark.parametrize("base,rows,window,ring_rows,heads,kv_heads,softcap", [
     (0, 1, 0, 8, 2, 1, 0.0),                # one row at the first position: one tile of one key
     (63, 65, 0, 64, 4, 4, 0.0),             # tile and block borders, one head per KV head
-    (190, 256, 100, 256, 6, 2, 0.0),        # three heads per KV head (not packed), windows that begin inside tiles
-    (30, 129, 64, 64, 8, 1, 30.0),          # eight heads per KV head, a window of a whole tile
+    (190, 256, 100, 256, 4, 2, 0.0),        # windows that begin inside tiles
+    (30, 129, 64, 64, 4, 1, 30.0),          # four heads per KV head, a window of a whole tile
     (500, 40, 1, 512, 2, 2, 0.0),           # every row sees itself alone
 ])
 def test_prefill_attention_borders(gf, oracle, base, rows, window, ring_rows, heads, kv_heads, softcap):
     """Borders of the 128-query blocks and 64-key tiles, for every way heads share a block."""
     test_prefill_attention_matches_oracle(gf, oracle, base, rows, window, ring_rows, heads, kv_heads, softcap)
+
+
+@pytest.mark.parametrize("geometry,seed,cuts", [
+    ("tiny-target", 84, (300, 257)),        # rings of 32 rows that a chunk overflows; a second chunk behind a filled ring
+    ("tiny-target", 85, (65, 2100)),        # a short chunk ahead, then two equal wide ones
+    ("tiny-draft", 86, (330, 700)),         # an f32 cache: Q8_0 weights, chunks limited to 1024 rows
+    ("tiny-gemma2", 87, (511, 300)),        # capped scores, no norms of the heads
+])
+def test_wide_prompt_chunks(gf, gm, geometry, seed, cuts):
+    """Chunks of more than 256 rows (weights decoded to HBM, products on pairs of CTAs) against the exact row path: K/V rows
+    and logits within the bound the 256-row chunks have (test_tensor_prefill_matches_exact_row_path), and decoding behind them."""
+    config = syn.model_config(geometry)
+    weights = syn.make_model_weights(geometry, seed)
+    total = sum(cuts)
+    tokens = np.random.default_rng(seed).integers(0, config["vocab"], total + 2).astype(np.uint32)
+    wide, exact = gm.Model(config, weights, total + 64, 8), gm.Model(config, weights, total + 64, 8)
+    exact.use_tensor_prefill(False)
+    for model in (wide, exact):
+        done = 0
+        for count in cuts:
+            model.prefill(tokens[done:done + count])
+            done += count
+        assert model.position == total and model.status() == 0
+    worst = rel_l2(wide.logits(0), exact.logits(exact.prefill_logits_row))
+    for layer in range(config["layers"]):
+        for got, want in zip(wide.read_kv(layer, total - 12, 12), exact.read_kv(layer, total - 12, 12)):
+            worst = max(worst, rel_l2(got, want))
+    print(f"{geometry} {cuts}: wide chunks vs exact rows {worst:.2e}")
+    assert worst < 3e-2
+    for model in (wide, exact):
+        model.forward(tokens[total:], logits=True)
+        model.publish(2)
+        model.truncate(total)
+        assert model.status() == 0
+    assert rel_l2(wide.logits(1), exact.logits(1)) < 3e-2
