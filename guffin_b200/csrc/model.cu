@@ -453,6 +453,7 @@ int Model::reset() {
     if (matmul_counters_bytes_) GF_CUDA(cudaMemsetAsync(matmul_counters_, 0, matmul_counters_bytes_, stream_));
     if (attention_ws_) GF_CUDA(cudaMemsetAsync(attention_counters(attention_ws_, config_.row_capacity, config_.heads), 0,
                             (size_t)config_.row_capacity * config_.heads * sizeof(uint32_t), stream_));
+    if (wide_.counters) GF_CUDA(cudaMemsetAsync(wide_.counters, 0, wide_.counter_bytes, stream_));
     if (head_counters_) GF_CUDA(cudaMemsetAsync(head_counters_, 0, 2u * (config_.heads + 2u * config_.kv_heads) * sizeof(uint32_t), stream_));
     if (layered_ && layered_->counters) {
         uint32_t heads = 0;
@@ -1105,13 +1106,17 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
     return GF_OK;
 }
 
-// Decoding all weights to HBM costs a chunk the same whatever its rows, so it pays from a number of rows on (kWideFrom);
-// prompts are cut into equal chunks.  Shards keep the 256-row chunks (their exchange is laid out for those), as do plans
-// whose heads prefill_attention_supported refuses; an f32 cache limits the rows to what the row kernels' workspace allows.
-constexpr uint32_t kWideFrom = 257;
+// Prompts are cut into equal chunks of up to 2048 rows.  Up to kPackedRows rows decode weights on the way to the tensor core,
+// longer chunks once to HBM (which costs a 9B plan 4 ms whatever the rows: 257 rows take 11.6 ms the one way, 258 16.2 the
+// other, two short chunks as much).  Shards keep prefill_chunk (their exchange is laid out for its 256-row chunks), as do plans whose heads
+// prefill_attention_supported refuses and chunks of up to 128 rows of a plan with an f32 cache, whose matrices are so small
+// that its 128-row products are ahead (270M plan, 99 rows: 1.97 against 2.07 ms; 191 rows: 2.50 against 2.41).  An f32 cache
+// limits the rows to what the row kernels' workspace allows.
+constexpr uint32_t kWideFrom = 64, kWideFromF32 = 129;
 uint32_t Model::wide_rows(uint32_t left) const {
     const gf_model_config& c = config_;
-    if (left < kWideFrom || sharded() || c.head_dim != 256u || !caches_[0].rope_rotation) return 0;
+    const uint32_t from = c.kv_f16 ? kWideFrom : kWideFromF32;
+    if (left < from || sharded() || c.head_dim != 256u || !caches_[0].rope_rotation) return 0;
     const uint32_t group = c.heads / c.kv_heads;
     if (group != 1u && group != 2u && group != 4u) return 0;
     for (const LayerWeights& w : layers_)
@@ -1119,7 +1124,7 @@ uint32_t Model::wide_rows(uint32_t left) const {
             if (m->n % kPrefillTile || m->k % 128u) return 0;
     uint32_t most = std::min(kWideRows, (c.context + 15u) & ~15u);
     if (!c.kv_f16) most = std::min(most, 4096u / c.heads);
-    if (most < kWideFrom) return 0;
+    if (most < from) return 0;
     const uint32_t chunks = (left + most - 1u) / most;
     return (left + chunks - 1u) / chunks;
 }
@@ -1158,18 +1163,29 @@ int Model::ensure_wide_arena() {
     const size_t row = cache_row_bytes(0);
     GF_TRY(device_alloc(allocations_, &bytes, row * rows)); a.own_k = bytes;
     GF_TRY(device_alloc(allocations_, &bytes, row * rows)); a.own_v = bytes;
-    size_t tiles = 0;
-    for (const LayerWeights& w : layers_) {
-        auto total = [](std::initializer_list<const PackedMatrix*> set) { size_t n = 0; for (const PackedMatrix* m : set) n += (size_t)m->n * m->k * 2u; return n; };
-        tiles = std::max({tiles, total({&w.q, &w.k, &w.v}), total({&w.o}), total({&w.gate, &w.up}), total({&w.down})});
-    }
-    GF_TRY(device_alloc(allocations_, &a.tiles, tiles));
+    GF_TRY(device_alloc(allocations_, &bytes, packed_partial_bytes()));
+    a.partial = reinterpret_cast<float*>(bytes);
+    const size_t tiles = 2u * (std::max<size_t>({2u * c.ffn, qw + 2u * kvw, c.hidden}) / 128u + 1u);      // two counts each
+    GF_TRY(device_alloc(allocations_, &a.counters, tiles));
+    a.counter_bytes = tiles * sizeof(uint32_t);
+    GF_CUDA(cudaMemsetAsync(a.counters, 0, a.counter_bytes, stream_));
     GF_TRY(device_alloc(allocations_, &a.tokens, rows));
     a.rows = rows;
     return GF_OK;
 }
 
-// One wide chunk.  A layer is: norm; decode and multiply Q, K, V; rotation and cache rows; attention; decode and multiply O;
+// The decoded weights of a launch, for chunks that decode them to HBM.
+int Model::ensure_wide_tiles() {
+    if (wide_.tiles) return GF_OK;
+    size_t tiles = 0;
+    for (const LayerWeights& w : layers_) {
+        auto total = [](std::initializer_list<const PackedMatrix*> set) { size_t n = 0; for (const PackedMatrix* m : set) n += (size_t)m->n * m->k * 2u; return n; };
+        tiles = std::max({tiles, total({&w.q, &w.k, &w.v}), total({&w.o}), total({&w.gate, &w.up}), total({&w.down})});
+    }
+    return device_alloc(allocations_, &wide_.tiles, tiles);
+}
+
+// One such chunk.  A layer is: norm; decode and multiply Q, K, V; rotation and cache rows; attention; decode and multiply O;
 // norm; decode gate and up side by side and multiply with the gate in the output; decode and multiply down.  Norms and
 // products are those of a layered plan's chunks.
 int Model::prefill_wide(const uint32_t* tokens_host, uint32_t rows) {
@@ -1189,6 +1205,24 @@ int Model::prefill_wide(const uint32_t* tokens_host, uint32_t rows) {
     };
     // Matrices behind one another in the tile buffer, or two of equal shape with their groups of eight columns in turn.
     auto multiply = [&](std::initializer_list<const PackedMatrix*> set, bool paired, const Operand& in, std::initializer_list<float*> outs, const Operand* result) -> int {
+        bool one_family = true;
+        for (const PackedMatrix* m : set) one_family = one_family && unit_elements(m->dtype) == unit_elements((*set.begin())->dtype);
+        if (rows <= kPackedRows && one_family) {
+            PackedProduct product;
+            auto out = outs.begin();
+            for (const PackedMatrix* m : set) {
+                PackedProduct::Matrix& to = product.m[product.matrices++];
+                to.packed = m->data; to.dtype = (uint32_t)m->dtype; to.n = (uint32_t)m->n;
+                if (!paired) to.out = *out++;
+                product.k = (uint32_t)m->k;
+            }
+            product.rows = rows; product.paired = paired; product.a = in;
+            if (paired) product.result = *result;
+            product.partial = a.partial; product.counters = a.counters; product.error_flag = error_flag_;
+            ++launches_;
+            return launch_packed_product(product, stream_);
+        }
+        GF_TRY(ensure_wide_tiles());
         WideDecode decode;
         ChunkProduct product;
         product.problems = 0; product.rows = rows; product.error_flag = error_flag_;

@@ -259,6 +259,7 @@ private:
     // Wide prompt chunks (prompt.cuh): how many of the `left` rows of a prompt the next one takes, 0 for none.
     uint32_t wide_rows(uint32_t left) const;
     int ensure_wide_arena();
+    int ensure_wide_tiles();
     int prefill_wide(const uint32_t* tokens_host, uint32_t rows);
     struct WideArena {
         uint32_t rows = 0;                                   // at most, per chunk; 0: not allocated
@@ -266,7 +267,10 @@ private:
         float *residual = nullptr, *projected = nullptr, *raw_q = nullptr, *raw_k = nullptr, *raw_v = nullptr, *query32 = nullptr;
         __half* query = nullptr;
         void *own_k = nullptr, *own_v = nullptr;             // one layer's cache rows of a chunk
-        uint8_t* tiles = nullptr;                            // the decoded weights of one launch
+        uint8_t* tiles = nullptr;                            // the decoded weights of one launch (chunks beyond kPackedRows)
+        float* partial = nullptr;                            // pieces of tiles cut between CTAs, and their arrival counts
+        uint32_t* counters = nullptr;
+        size_t counter_bytes = 0;
         void* attention_ws = nullptr;                        // f32 caches
         float* attention_out = nullptr;
         uint32_t* tokens = nullptr;

@@ -1,8 +1,8 @@
 // Prompt chunks of up to kWideRows rows of a quantised plan: a launch's weights are decoded to bf16 tiles in HBM once and
 // multiplied with all rows of the chunk by the product kernel of the layered plans (dense_prefill.cu), norms, rotation and
-// gate fused around it (Model::prefill_wide, model.cu).  Shorter chunks keep prefill.cu's kernel, which decodes in shared
-// memory.  2048 tokens into the 12B plan: 131.8 ms in chunks of 256 rows (that kernel is bound by decoding), 45.2 ms in one
-// of 2048; 777 tokens into the 270M plan 5.1 -> 3.3 ms.
+// gate fused around it (Model::prefill_wide, model.cu).    2048 tokens into the 12B plan: 131.8 ms in chunks of 256 rows (that kernel is bound by decoding), 45.2 ms in one
+// of 2048; 777 tokens into the 270M plan 5.1 -> 3.3 ms.  (prefill.cu's kernel is left to shards and to short chunks of plans
+// with an f32 cache.)
 #pragma once
 
 #include "dense.cuh"
@@ -25,6 +25,25 @@ struct WideDecode {
 };
 // The reference's values exactly, then one rounding to bf16 (as prefill.cu's kernel decodes them).
 int launch_wide_decode(const WideDecode& decode, cudaStream_t stream);
+
+// Chunks of up to kPackedRows rows instead decode a launch's weights on their way to the tensor core (packed_product.cu).
+constexpr uint32_t kPackedRows = 256;
+struct PackedProduct {
+    struct Matrix {
+        const uint8_t* packed = nullptr;
+        float* out = nullptr;                    // [rows][n]; not used by a pair
+        uint32_t dtype = 0, n = 0, first_tile = 0;
+    } m[3];
+    uint32_t matrices = 0, rows = 0, k = 0;
+    bool paired = false;                         // two matrices of one shape: result(row, n) = gelu(m[0]) * m[1]
+    Operand a, result;
+    float* partial = nullptr;                    // packed_partial_bytes()
+    uint32_t* counters = nullptr;                // two per 128 columns of the launch, zero between launches
+    int* error_flag = nullptr;
+    uint32_t tiles = 0, units = 0, unit_elems = 0, n_rows = 0, row_bytes = 0, stages = 0, unit_slots = 0;      // filled by the launcher
+};
+size_t packed_partial_bytes();
+int launch_packed_product(PackedProduct product, cudaStream_t stream);
 
 // Per-head norm (skipped without weights), rotation from the table, and the cache rows: q [rows][heads * 256] f16
 // multiplied by `scale` (or f32 as it is, with q32), keys and values [rows][kv_heads * 256] f16 or f32.

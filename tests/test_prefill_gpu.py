@@ -141,9 +141,12 @@ def test_prefill_attention_borders(gf, oracle, base, rows, window, ring_rows, he
     ("tiny-target", 85, (65, 2100)),        # a short chunk ahead, then two equal wide ones
     ("tiny-draft", 86, (330, 700)),         # an f32 cache: Q8_0 weights, chunks limited to 1024 rows
     ("tiny-gemma2", 87, (511, 300)),        # capped scores, no norms of the heads
+    ("tiny-target", 88, (66, 97, 257)),     # chunks of up to 256 rows, decoded on their way to the tensor core: the shortest,
+    ("tiny-draft", 89, (225, 130)),         # products of 96, 128, 160, 224 and 256 rows
+    ("tiny-gemma2", 90, (161, 193)),
 ])
 def test_wide_prompt_chunks(gf, gm, geometry, seed, cuts):
-    """Chunks of more than 256 rows (weights decoded to HBM, products on pairs of CTAs) against the exact row path: K/V rows
+    """Chunks of more than 256 rows (weights decoded to HBM, products on pairs of CTAs) and shorter ones against the exact row path: K/V rows
     and logits within the bound the 256-row chunks have (test_tensor_prefill_matches_exact_row_path), and decoding behind them."""
     config = syn.model_config(geometry)
     weights = syn.make_model_weights(geometry, seed)
@@ -169,3 +172,24 @@ def test_wide_prompt_chunks(gf, gm, geometry, seed, cuts):
         model.truncate(total)
         assert model.status() == 0
     assert rel_l2(wide.logits(1), exact.logits(1)) < 3e-2
+
+
+@pytest.mark.parametrize("geometry,ffn,rows", [("tiny-target", 16384, 66), ("tiny-target", 20736, 200), ("tiny-draft", 24576, 131)])
+def test_tiles_cut_between_ctas(gf, gm, geometry, ffn, rows):
+    """A down projection of few columns and long K, whose tiles are cut along K and added from pieces, and gate and up
+    products of more tiles than SMs, some of them cut: K/V rows and logits against the exact row path, twice in a row."""
+    config = dict(syn.model_config(geometry), ffn=ffn, layers=2)
+    weights = syn.make_model_weights(geometry, 91, config)
+    tokens = np.random.default_rng(91).integers(0, config["vocab"], rows + 1).astype(np.uint32)
+    tensor, exact = gm.Model(config, weights, rows + 32, 8), gm.Model(config, weights, rows + 32, 8)
+    exact.use_tensor_prefill(False)
+    exact.prefill(tokens)
+    for _ in range(2):
+        tensor.reset()
+        tensor.prefill(tokens)
+        assert tensor.status() == 0
+        worst = rel_l2(tensor.logits(0), exact.logits(exact.prefill_logits_row))
+        for layer in range(2):
+            for got, want in zip(tensor.read_kv(layer, rows - 8, 8), exact.read_kv(layer, rows - 8, 8)):
+                worst = max(worst, rel_l2(got, want))
+        assert worst < 3e-2
