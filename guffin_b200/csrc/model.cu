@@ -1009,6 +1009,22 @@ int Model::ensure_prefill_arena() {
 // One chunk of up to 128 prompt rows: every projection is one tensor-core GEMM over all rows of the
 // chunk; norms, GeGLU and the attention output go through small kernels that write the next GEMM's bf16
 // operand; RoPE / K/V store and attention reuse the row kernels.  The rows are published at the end.
+// A shard's O and down products are partial sums: the chunk's rows are summed over the shards in one launch.
+int Model::exchange_chunk(float* x, uint32_t rows, uint32_t& splits, uint32_t half, uint32_t site) {
+    const ShardExchange& shards = shard_;
+    ShardBulk bulk {};
+    bulk.x = x; bulk.splits = splits; bulk.slab = kPrefillRows * config_.hidden; bulk.values = rows * config_.hidden;
+    bulk.shards = shards.size; bulk.self = shards.rank; bulk.peers = 0;
+    for (uint32_t s = 0; s < shards.size; ++s) {
+        bulk.parts[s] = shards.part(shards.arena, half, s);
+        if (s != shards.rank) bulk.out[bulk.peers++] = shards.part(shards.mapped[s], half, shards.rank);
+    }
+    bulk.tick = shards.tick(); bulk.site = site; bulk.wait_limit = shards.wait_limit; bulk.error_flag = error_flag_;
+    splits = 1;
+    ++launches_;
+    return launch_shard_bulk_exchange(bulk, stream_);
+}
+
 int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
     const gf_model_config& c = config_;
     PrefillArena& a = prefill_;
@@ -1019,21 +1035,6 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
     launches_ += 1;
     const bool fused_exchange = shard_.connected;
     if (fused_exchange) { ++launches_; GF_TRY(launch_shard_tick(shard_.tick(), stream_)); }
-    // A shard's O and down products are partial sums: the chunk's rows are summed over the shards in one launch.
-    auto exchange = [&](uint32_t& splits, uint32_t half, uint32_t site) -> int {
-        const ShardExchange& x = shard_;
-        ShardBulk bulk {};
-        bulk.x = a.projected; bulk.splits = splits; bulk.slab = kPrefillRows * c.hidden; bulk.values = rows * c.hidden;
-        bulk.shards = x.size; bulk.self = x.rank; bulk.peers = 0;
-        for (uint32_t s = 0; s < x.size; ++s) {
-            bulk.parts[s] = x.part(x.arena, half, s);
-            if (s != x.rank) bulk.out[bulk.peers++] = x.part(x.mapped[s], half, x.rank);
-        }
-        bulk.tick = x.tick(); bulk.site = site; bulk.wait_limit = x.wait_limit; bulk.error_flag = error_flag_;
-        splits = 1;
-        ++launches_;
-        return launch_shard_bulk_exchange(bulk, stream_);
-    };
     auto gemm = [&](std::initializer_list<std::pair<const PackedMatrix*, float*>> set, const void* operand, uint64_t k, uint32_t splits = 1) -> int {
         PrefillGemmLaunch launch;
         launch.count = 0;
@@ -1083,7 +1084,7 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
         GF_TRY(launch_prefill_pack(a.attention_out, a.a_q, rows, qw, stream_));
         uint32_t o_splits = prefill_gemm_splits(w.o.n, w.o.k, w.o.dtype);
         GF_TRY(gemm({{&w.o, a.projected}}, a.a_q, qw, o_splits));
-        if (fused_exchange) GF_TRY(exchange(o_splits, 0u, 2u * l + 1u));
+        if (fused_exchange) GF_TRY(exchange_chunk(a.projected, rows, o_splits, 0u, 2u * l + 1u));
         GF_TRY(launch_prefill_norm(a.projected, o_splits, a.residual, w.post_attention_norm, w.ffn_norm, a.residual2, a.a_hidden, rows, c.hidden,
                                    c.rms_eps, 1, stream_));
         uint32_t ffn_splits = 1;
@@ -1097,7 +1098,7 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
         GF_TRY(launch_prefill_geglu(a.gate, a.up, ffn_splits, a.a_ffn, rows, c.ffn, stream_));
         down_splits = prefill_gemm_splits(w.down.n, w.down.k, w.down.dtype);
         GF_TRY(gemm({{&w.down, a.projected}}, a.a_ffn, c.ffn, down_splits));
-        if (fused_exchange) GF_TRY(exchange(down_splits, 1u, 2u * l + 2u));
+        if (fused_exchange) GF_TRY(exchange_chunk(a.projected, rows, down_splits, 1u, 2u * l + 2u));
         launches_ += 5;
     }
     GF_TRY(launch_kv_publish(a.publish_layers, c.layers, state_dev_, rows, stream_));
@@ -1108,15 +1109,14 @@ int Model::prefill_chunk(const uint32_t* tokens_host, uint32_t rows) {
 
 // Prompts are cut into equal chunks of up to 2048 rows.  Up to kPackedRows rows decode weights on the way to the tensor core,
 // longer chunks once to HBM (which costs a 9B plan 4 ms whatever the rows: 257 rows take 11.6 ms the one way, 258 16.2 the
-// other, two short chunks as much).  Shards keep prefill_chunk (their exchange is laid out for its 256-row chunks), as do plans whose heads
-// prefill_attention_supported refuses and chunks of up to 128 rows of a plan with an f32 cache, whose matrices are so small
+// other, two short chunks as much).  prefill_chunk is left to plans whose heads prefill_attention_supported refuses and to chunks of up to 128 rows of a plan with an f32 cache, whose matrices are so small
 // that its 128-row products are ahead (270M plan, 99 rows: 1.97 against 2.07 ms; 191 rows: 2.50 against 2.41).  An f32 cache
 // limits the rows to what the row kernels' workspace allows.
 constexpr uint32_t kWideFrom = 64, kWideFromF32 = 129;
 uint32_t Model::wide_rows(uint32_t left) const {
     const gf_model_config& c = config_;
     const uint32_t from = c.kv_f16 ? kWideFrom : kWideFromF32;
-    if (left < from || sharded() || c.head_dim != 256u || !caches_[0].rope_rotation) return 0;
+    if (left < from || (sharded() && !shard_.connected) || c.head_dim != 256u || !caches_[0].rope_rotation) return 0;
     const uint32_t group = c.heads / c.kv_heads;
     if (group != 1u && group != 2u && group != 4u) return 0;
     for (const LayerWeights& w : layers_)
@@ -1124,6 +1124,7 @@ uint32_t Model::wide_rows(uint32_t left) const {
             if (m->n % kPrefillTile || m->k % 128u) return 0;
     uint32_t most = std::min(kWideRows, (c.context + 15u) & ~15u);
     if (!c.kv_f16) most = std::min(most, 4096u / c.heads);
+    if (sharded()) most = std::min(most, kPrefillRows);                // the rows the exchange is laid out for
     if (most < from) return 0;
     const uint32_t chunks = (left + most - 1u) / most;
     return (left + chunks - 1u) / chunks;
@@ -1196,6 +1197,9 @@ int Model::prefill_wide(const uint32_t* tokens_host, uint32_t rows) {
     GF_CUDA(cudaMemcpyAsync(a.tokens, tokens_host, rows * sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));      // pageable: staged by the driver
     GF_TRY(launch_embedding(token_embd_.dtype, token_embd_.data, c.hidden, token_vocab(), a.tokens, rows, sqrtf((float)c.hidden), a.residual, status_dev_, stream_, false));
     ++launches_;
+    const bool fused_exchange = shard_.connected;
+    uint32_t whole = 1;
+    if (fused_exchange) { ++launches_; GF_TRY(launch_shard_tick(shard_.tick(), stream_)); }
     ChunkNorm norm;
     norm.residual = a.residual; norm.width = c.hidden; norm.rows = rows; norm.eps = c.rms_eps; norm.result = a.hidden;
     auto normalise = [&](const float* y, const float* gain0, const float* gain1) -> int {
@@ -1300,9 +1304,11 @@ int Model::prefill_wide(const uint32_t* tokens_host, uint32_t rows) {
         }
         if (last) break;
         GF_TRY(multiply({&w.o}, false, a.heads, {a.projected}, nullptr));
+        if (fused_exchange) GF_TRY(exchange_chunk(a.projected, rows, whole, 0u, 2u * l + 1u));
         GF_TRY(normalise(a.projected, w.post_attention_norm, w.ffn_norm));
         GF_TRY(multiply({&w.gate, &w.up}, true, a.hidden, {}, &a.ffn));
         GF_TRY(multiply({&w.down}, false, a.ffn, {a.projected}, nullptr));
+        if (fused_exchange) GF_TRY(exchange_chunk(a.projected, rows, whole, 1u, 2u * l + 2u));
     }
     ++launches_;
     GF_TRY(launch_advance_position(state_dev_, rows, stream_));

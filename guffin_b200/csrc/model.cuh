@@ -260,6 +260,7 @@ private:
     uint32_t wide_rows(uint32_t left) const;
     int ensure_wide_arena();
     int ensure_wide_tiles();
+    int exchange_chunk(float* x, uint32_t rows, uint32_t& splits, uint32_t half, uint32_t site);
     int prefill_wide(const uint32_t* tokens_host, uint32_t rows);
     struct WideArena {
         uint32_t rows = 0;                                   // at most, per chunk; 0: not allocated

@@ -1,8 +1,7 @@
 // Prompt chunks of up to kWideRows rows of a quantised plan: a launch's weights are decoded to bf16 tiles in HBM once and
 // multiplied with all rows of the chunk by the product kernel of the layered plans (dense_prefill.cu), norms, rotation and
-// gate fused around it (Model::prefill_wide, model.cu).    2048 tokens into the 12B plan: 131.8 ms in chunks of 256 rows (that kernel is bound by decoding), 45.2 ms in one
-// of 2048; 777 tokens into the 270M plan 5.1 -> 3.3 ms.  (prefill.cu's kernel is left to shards and to short chunks of plans
-// with an f32 cache.)
+// gate fused around it (Model::prefill_wide, model.cu).  2048 tokens into the 12B plan: 131.8 ms in chunks of 256 rows of prefill.cu's
+// kernel (which decodes in shared memory), 45.2 ms in one of 2048; 777 tokens into the 270M plan 5.1 -> 3.3 ms.
 #pragma once
 
 #include "dense.cuh"
