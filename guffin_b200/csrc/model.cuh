@@ -34,7 +34,7 @@ struct LayerWeights {
 
 struct LayerCache {
     void *ring_k = nullptr, *ring_v = nullptr;        // [ring_rows][kv_width]
-    void *private_k = nullptr, *private_v = nullptr;  // [row_capacity][kv_width]
+    void *private_k = nullptr, *private_v = nullptr;  // [pass rows][kv_width]
     uint32_t ring_rows = 0;                           // power of two (gemma2_metal_plan.cpp:356-366)
     uint32_t window = 0;                              // 0 = global layer
     float rope_base = 0.0f, rope_scale = 1.0f;
@@ -85,6 +85,8 @@ public:
     int reset();
     int forward(const uint32_t* tokens_host, uint32_t rows, uint32_t flags);
     int publish(uint32_t rows);
+    int forward_rows(const uint32_t* tokens_host, uint32_t rows, uint32_t flags, uint32_t most);      // the same beyond row_capacity
+    int publish_rows(uint32_t rows, uint32_t most);
     int select(const void* requests_host, uint32_t rows);
     int read_candidates(void* results_host, uint32_t rows);
     int read_logits(uint32_t row, float* host);
@@ -339,6 +341,8 @@ private:
     void* requests_pinned_ = nullptr;
     uint32_t position_ = 0;
     uint32_t launches_ = 0;
+    uint32_t pass_rows_ = 0;                                 // rows of a prompt's passes; 0 on a layered plan
+    uint32_t buffer_rows() const { return pass_rows_ ? (uint32_t)GF_MAX_ROWS : config_.row_capacity; }      // rows the pass buffers hold
     cudaGraphExec_t graphs_[GF_MAX_ROWS + 1][2] = {};
     uint32_t graph_launches_[GF_MAX_ROWS + 1][2] = {};      // kernel nodes of each recorded graph
     // Decode pass kernel: recorded tables per (rows, logits), one for the weight sweep per rows.

@@ -210,8 +210,8 @@ int Model::encode_stream_group(StreamSet& set, uint32_t first, uint32_t rows) {
         ap.q = query_; ap.ring_k = nullptr; ap.ring_v = nullptr; ap.private_k = cache.private_k; ap.private_v = cache.private_v;
         ap.out = attention_out_;
         ap.partial_out = static_cast<float*>(attention_ws_);
-        ap.partial_ml = ap.partial_out + (size_t)c.row_capacity * c.heads * kMaxAttentionPartitions * 256u;
-        ap.counters = attention_counters(attention_ws_, c.row_capacity, c.heads);
+        ap.partial_ml = ap.partial_out + (size_t)buffer_rows() * c.heads * kMaxAttentionPartitions * 256u;
+        ap.counters = attention_counters(attention_ws_, buffer_rows(), c.heads);
         ap.base_position = positions; ap.rows = rows; ap.heads = c.heads; ap.kv_heads = c.kv_heads; ap.head_dim = c.head_dim;
         ap.ring_mask = cache.ring_rows - 1u; ap.window = cache.window; ap.scale = c.attention_scale;
         ap.softcap = c.attn_softcap; ap.kv_f16 = c.kv_f16;

@@ -193,3 +193,28 @@ def test_tiles_cut_between_ctas(gf, gm, geometry, ffn, rows):
             for got, want in zip(tensor.read_kv(layer, rows - 8, 8), exact.read_kv(layer, rows - 8, 8)):
                 worst = max(worst, rel_l2(got, want))
         assert worst < 3e-2
+
+
+@pytest.mark.parametrize("geometry,row_capacity,count", [("tiny-target", 1, 9), ("tiny-target", 2, 10), ("tiny-target", 3, 47),
+                                                         ("tiny-draft", 2, 64), ("tiny-gemma2", 8, 33)])
+def test_short_prompts_in_wide_passes(gf, gm, geometry, row_capacity, count):
+    """A prompt too short for chunks runs in passes of eight rows whatever the plan's passes hold, the last pass in the
+    plan's own: cache rows, logits and the last pass taken back and run again, against tokens given one by one.  Products do not
+    depend on the rows of a pass; the attention's partitions do, by f32 roundings that binary16 cache rows (2^-11) amplify."""
+    config = syn.model_config(geometry)
+    weights = syn.make_model_weights(geometry, 92)
+    tokens = np.random.default_rng(92).integers(0, config["vocab"], count).astype(np.uint32)
+    plan, single = gm.Model(config, weights, 80, row_capacity), gm.Model(config, weights, 80, 1)
+    plan.prefill(tokens)
+    for token in tokens:
+        single.forward(np.array([token], np.uint32), logits=True)
+        single.publish(1)
+    assert plan.position == count and plan.status() == 0
+    assert plan.prefill_logits_row < row_capacity
+    assert rel_l2(plan.logits(plan.prefill_logits_row), single.logits(0)) < 2e-3
+    for layer in range(config["layers"]):
+        for got, want in zip(plan.read_kv(layer, count - 8, 8), single.read_kv(layer, count - 8, 8)):
+            assert rel_l2(got, want) < 2e-3
+    plan.truncate(count - row_capacity)
+    plan.forward(tokens[count - row_capacity:], logits=True)
+    assert rel_l2(plan.logits(row_capacity - 1), single.logits(0)) < 2e-3
