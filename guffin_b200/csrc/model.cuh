@@ -270,7 +270,11 @@ private:
         float *residual = nullptr, *projected = nullptr, *raw_q = nullptr, *raw_k = nullptr, *raw_v = nullptr, *query32 = nullptr;
         __half* query = nullptr;
         void *own_k = nullptr, *own_v = nullptr;             // one layer's cache rows of a chunk
-        uint8_t* tiles = nullptr;                            // the decoded weights of one launch (chunks beyond kPackedRows)
+        // Chunks beyond kPackedRows: the decoded weights of two launches in turn, decoded on a stream of their own.
+        uint8_t* tiles[2] = {nullptr, nullptr};
+        cudaStream_t decode_stream = nullptr;
+        cudaEvent_t decoded[2] = {nullptr, nullptr}, multiplied[2] = {nullptr, nullptr};
+        uint32_t turn = 0;
         float* partial = nullptr;                            // pieces of tiles cut between CTAs, and their arrival counts
         uint32_t* counters = nullptr;
         size_t counter_bytes = 0;
